@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster(const SelectArgs
     const uint32_t tail_bits = (n_s & 31) ? (1u << (n_s & 31)) - 1u : 0xffffffffu;
     if (!a.masks)
         for (int w = tid; w < a.slice_len / 32; w += NT) eff[w] = w < words ? (w == words - 1 ? tail_bits : 0xffffffffu) : 0u;
+    cluster.barrier_arrive();  // (waited for before the first store into another CTA: by then all sixteen have started)
     __syncthreads();
     // Launched with programmatic stream serialisation: nothing is read from global memory before the previous
     // kernel of the stream has finished; what precedes this line overlaps its tail.
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster(const SelectArgs
         const uint32_t holders = __ballot_sync(kFull, w == w1);
         if (lane == __ffs(holders) - 1) w = 0u;
         const uint32_t w2 = __reduce_max_sync(kFull, w);
+        cluster.barrier_wait();
         // every CTA receives the witnesses (lane l stores into CTA l / 2): the bound search then reads its own memory
         cluster.map_shared_rank(&cs, lane >> 1)->wit[(rank * kWarps + warp) * 2 + (lane & 1)] = (lane & 1) ? w2 : w1;
     }

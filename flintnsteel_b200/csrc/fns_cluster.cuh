@@ -39,6 +39,9 @@ struct ClusterShared {
     uint32_t local_bound[kClusterCtas];  // second chance: the bound that each CTA could make of its own threads' maxima
     __align__(16) uint32_t wit[kClusterCtas * 16];  // the witnesses, two per warp of the cluster (every CTA gets a copy)
 };
+// One fp32 session of V = 151,936 with 4,096 history ids (what Sampler and Engine have by default) leaves 320 bytes of the
+// 112 KB that a CTA may have.  Past them the call falls to k_select in slices: 21 us instead of 8.5.
+static_assert(sizeof(ClusterShared) <= 2560, "k_cluster would lose calls to k_select");
 
 template <typename T>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster(const SelectArgs a) {
@@ -273,13 +276,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster(const SelectArgs
 
     // 4. the bound: (nearly) the k-th largest witness, which every CTA finds in its own copy of the witnesses
     int reach;
-    uint32_t bound = block_reach<NT>([&](int i) { return cs.wit[i]; }, NT, k, 4, sh.sc, &reach);
+    uint32_t bound = block_reach<NT>([&](int i) { return cs.wit[i]; }, NT, k, 4, sh.sc, sh.ends, &reach);
     if (bound == 0u) {  // (the same in every CTA: all searched the same witnesses)
         // Fewer than k witnesses.  Under a mask whose allowed ids lie in a few slices that is no proof that the row has
         // fewer than k candidates: a CTA whose own threads hold k maxima makes a bound of them, every CTA gets every
         // such bound, and the largest is the row's.  (Two warps' witnesses per CTA were all that it could send above.)
         __syncthreads();
-        const uint32_t mine = block_reach<NT>([&](int) { return tmax > -INFINITY ? order_word(tmax) : 0u; }, NT, k, 4, sh.sc, &reach);
+        const uint32_t mine = block_reach<NT>([&](int) { return tmax > -INFINITY ? order_word(tmax) : 0u; }, NT, k, 4, sh.sc, sh.ends, &reach);
         if (tid < kClusterCtas) cluster.map_shared_rank(&cs, tid)->local_bound[rank] = mine;
         cluster.sync();
 #pragma unroll
@@ -523,7 +526,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_cluster(const SelectArgs
         const uint32_t before = __shfl_sync(kFull, n_upto, r) - cnt;
         for (uint32_t i = (uint32_t) (tid & 15); i < cnt; i += 16u) lbuf[before + i] = gbuf[(size_t) r * kClusterRegion + i];
         __syncthreads();
-        const uint64_t * keys = cut_keys<NT>(lbuf, &n, k, gbuf, gsel, sh.sc);
+        const uint64_t * keys = cut_keys<NT>(lbuf, &n, k, gbuf, gsel, sh);
         rank_draw<NT>(keys, n, k, sorted, pj, acc, reinterpret_cast<double *>(gsel), sh.sc, p, sh.u01, sh.inv_t, a.k_cap, tok, oc);
     }
 }

@@ -124,7 +124,6 @@ struct SelectScratch {
     uint32_t hist[256];
     uint32_t or_hi, or_lo, and_hi, and_lo;
     uint32_t bucket, need, bucket_count, count;
-    __align__(16) uint32_t ends[64];  // block_reach: the warps' largest and smallest words
 };
 
 // tau such that exactly min(k, n) of the DISTINCT, NON-ZERO keys buf[0 .. n) are >= tau (0 when n <= k).
@@ -227,10 +226,10 @@ __device__ uint64_t block_kth_key(const uint64_t * buf, int n, int k, SelectScra
 // than k others are there.  One histogram of 256 bins between the smallest and the largest word, whose pivot bin is split
 // again until it is fine enough - usually at once; every warp reads the bins for itself, so a pass is two block barriers.
 // (256 witnesses: 0.4 us; one warp deciding two bits per step by warp-wide counts took 0.9 us.)
-// word(i) is only called by thread i % NT.  All NT threads with uniform arguments; the block must be synchronised before
-// sc is used again.
+// word(i) is only called by thread i % NT.  `ends` has room for two words per warp.  All NT threads with uniform arguments;
+// the block must be synchronised before sc or ends is used again.
 template <int NT, typename F>
-__device__ __forceinline__ uint32_t block_reach(F word, int n, int k, int slack, SelectScratch & sc, int * reach) {
+__device__ __forceinline__ uint32_t block_reach(F word, int n, int k, int slack, SelectScratch & sc, uint32_t * ends, int * reach) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t hi = 0u, lo = 0xffffffffu;
     for (int i = tid; i < n; i += NT) {
@@ -242,13 +241,13 @@ __device__ __forceinline__ uint32_t block_reach(F word, int n, int k, int slack,
     hi = __reduce_max_sync(kFull, hi);
     lo = __reduce_min_sync(kFull, lo);
     if (lane == 0) {
-        sc.ends[warp] = hi;
-        sc.ends[32 + warp] = lo;
+        ends[warp] = hi;
+        ends[NT / 32 + warp] = lo;
     }
     for (int i = tid; i < 256; i += NT) sc.hist[i] = 0u;
     __syncthreads();
-    hi = __reduce_max_sync(kFull, lane < NT / 32 ? sc.ends[lane] : 0u);
-    lo = __reduce_min_sync(kFull, lane < NT / 32 ? sc.ends[32 + lane] : 0xffffffffu);
+    hi = __reduce_max_sync(kFull, lane < NT / 32 ? ends[lane] : 0u);
+    lo = __reduce_min_sync(kFull, lane < NT / 32 ? ends[NT / 32 + lane] : 0xffffffffu);
     *reach = 0;
     if (hi == 0u) return 0u;
     int bits = hi == lo ? 1 : 32 - __clz((int) (hi ^ lo));  // undecided bits

@@ -48,6 +48,7 @@ struct RowsShared {
     __align__(16) uint32_t wit[256];     // the row's witnesses (every CTA gets a copy)
     uint32_t hl_pos[kRowsThreads];       // the list: positions f
     float hl_raw[kRowsThreads];          // ... and logits
+    __align__(16) uint32_t lut[64];      // fill_or_masks
 };
 
 // A 16-byte load that happens only if `wanted` is not 0 (then r is replaced).  Written as one predicated instruction: with
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
     for (int i = tid; i < TS; i += NT) tkey[i] = kNoKey;
     if (listed)  // places that no segment takes name a segment behind the slice, whose bits are 0
         for (int i = tid; i < a.list_cap; i += NT) seglist[i] = (uint16_t) (a.slice_len / (32 * VEC));
-    fill_or_masks<T>(sh.lut);
+    fill_or_masks<T>(rs.lut);
     if (a.own_cap > 0)
         for (int i = tid * 4; i < eff_words; i += NT * 4) *reinterpret_cast<uint4 *>(hb + i) = make_uint4(0u, 0u, 0u, 0u);
     if (C > 1) cluster.barrier_arrive();  // (waited for before the first store into another CTA: by then all have started)
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
         if (bits) {
             if (bits != kCellBits) {  // excluded elements become NaN, which never wins (a vector not loaded holds old values)
 #pragma unroll
-                for (int u = 0; u < NV; ++u) exclude<T>(r[u], (bits >> (u * VEC)) & kVecBits, sh.lut);
+                for (int u = 0; u < NV; ++u) exclude<T>(r[u], (bits >> (u * VEC)) & kVecBits, rs.lut);
             }
             float even = -INFINITY;
 #pragma unroll
@@ -436,10 +437,10 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
     for (;;) {
         // 5. The bound.
         int reach;
-        uint32_t bound = block_reach<NT>([&](int i) { return rs.wit[i]; }, NT, witnesses, 4, sh.sc, &reach);
+        uint32_t bound = block_reach<NT>([&](int i) { return rs.wit[i]; }, NT, witnesses, 4, sh.sc, sh.ends, &reach);
         if (C > 1 && bound == 0u) {  // too few groups saw anything: the largest bound that a CTA can make alone
             __syncthreads();
-            const uint32_t mine = block_reach<NT>([&](int) { return wt; }, NT, witnesses, 4, sh.sc, &reach);
+            const uint32_t mine = block_reach<NT>([&](int) { return wt; }, NT, witnesses, 4, sh.sc, sh.ends, &reach);
             if (tid < C) cluster.map_shared_rank(&rs, tid)->local_bound[rank] = mine;
             cluster.sync();
             for (int r = 0; r < C; ++r) bound = max(bound, rs.local_bound[r]);
@@ -695,7 +696,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
         __syncthreads();
         keys = lbuf;
     }
-    keys = cut_keys<NT>(keys, &n_all, k, gbuf, sel, sh.sc);
+    keys = cut_keys<NT>(keys, &n_all, k, gbuf, sel, sh);
     rank_draw<NT>(keys, n_all, k, sorted, pj, acc, reinterpret_cast<double *>(sel), sh.sc, p, sh.u01, sh.inv_t, a.k_cap,
                   a.out_tokens ? a.out_tokens + row : nullptr, a.out_cands ? a.out_cands + (size_t) row * a.k_cap : nullptr);
 }

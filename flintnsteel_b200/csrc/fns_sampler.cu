@@ -93,11 +93,19 @@ struct SelectShared {
     uint32_t n_seg;       // segments with an allowed element
     int keep;
     int is_last;
-    __align__(16) float warp_bound[kMaxWarps];  // per warp: a value that r of its lanes have reached
-    uint32_t warp_top[kMaxWarps];               // per warp: its largest thread maximum (as an order word)
-    uint64_t red[kMaxWarps];
-    double u01, inv_t;    // the row's uniform and 1 / temperature
-    __align__(16) uint32_t lut[64];  // fill_or_masks
+    // (k_cluster's shared memory is sized to the last hundred bytes, and this is part of it: what two kernels need at
+    // different times shares its place)
+    union {
+        __align__(16) float warp_bound[kMaxWarps];  // per warp: a value that r of its lanes have reached
+        struct {
+            double u01, inv_t;                      // for the draw: the row's uniform and 1 / temperature
+        };
+    };
+    uint32_t warp_top[kMaxWarps];                   // per warp: its largest thread maximum (as an order word)
+    union {
+        uint64_t red[kMaxWarps];
+        uint32_t ends[2 * kMaxWarps];               // block_reach: the warps' largest and smallest words
+    };
 };
 
 __device__ __forceinline__ float to_float(float x) { return x; }
@@ -562,11 +570,12 @@ __device__ __forceinline__ void rank_draw(const uint64_t * buf, int n, int k, ui
 // All NT threads; block synchronised on entry and exit.
 constexpr int kCutMin = 192;
 template <int NT>
-__device__ __forceinline__ uint64_t * cut_keys(uint64_t * keys, int * n, int k, uint64_t * to, uint64_t * sel, SelectScratch & sc) {
+__device__ __forceinline__ uint64_t * cut_keys(uint64_t * keys, int * n, int k, uint64_t * to, uint64_t * sel, SelectShared & sh) {
+    SelectScratch & sc = sh.sc;
     const int have = *n;
     if (have <= k || have <= kCutMin) return keys;
     int reach;
-    const uint32_t bar = block_reach<NT>([&](int i) { return (uint32_t) (keys[i] >> 32); }, have, k, k >> 3, sc, &reach);
+    const uint32_t bar = block_reach<NT>([&](int i) { return (uint32_t) (keys[i] >> 32); }, have, k, k >> 3, sc, sh.ends, &reach);
     if (reach > kRankSelectMax) {
         __syncthreads();
         const uint64_t tau = block_kth_key<NT>(keys, have, k, sc);

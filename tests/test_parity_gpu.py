@@ -6,6 +6,7 @@ when the uniform lies within 1e-6 of a CDF boundary of the oracle's distribution
 libm exp may differ from CUDA's in the last bit).  Against the reference's kernels the tokens must be identical.
 """
 import ctypes
+import os
 
 import numpy as np
 import pytest
@@ -28,8 +29,10 @@ def dev():
 
 @pytest.fixture(scope="module")
 def ref():
-    from oracle.binding import RefGpu
+    from oracle.binding import REF_SO, RefGpu
 
+    if not os.path.exists(REF_SO):
+        pytest.skip(f"{REF_SO} is not built: it needs the reference tree (make -C oracle ref)")
     return RefGpu()
 
 

@@ -165,15 +165,19 @@ def test_compat_shim_grows_its_workspace(dev, library_path):
 
 def test_calls_can_be_captured_in_a_cuda_graph(dev, oracle):
     """The sampler is stream-ordered with no host synchronisation and no set-up left in the call path after
-    fns_b200_create, so a call can be captured and replayed: one row (sliced plan, tickets in the workspace), a
-    whole-row masked batch (k_select) and an unmasked batch (k_ring, bulk copies), each against its eager run."""
+    fns_b200_create, so a call can be captured and replayed: one row and nine rows
+    under masks (k_cluster), nine rows without (k_cluster), a batch of 40 under masks (k_rows, and k_select with its tickets
+    for k_cap 256), and 40 rows without (k_ring, bulk copies), each against its eager run."""
     from flintnsteel_b200.sampler import Sampler, params_to_device
 
     cases = [wl.grammar_row(seed=3), wl.session_batch(seed=5, rows=9, vocab=40_000, history=128),
              wl.session_batch(seed=6, rows=9, vocab=40_000, history=128)]
     cases[2].masks = None
+    cases += [wl.session_batch(seed=7 + i, rows=40, vocab=40_000, history=128) for i in range(3)]
+    cases[4].k_cap = 256
+    cases[5].masks = None
     for w in cases:
-        s = Sampler(0, max_rows=w.rows, max_vocab=w.vocab, k_cap=64, max_history=4096)
+        s = Sampler(0, max_rows=w.rows, max_vocab=w.vocab, k_cap=w.k_cap, max_history=4096)
         lg = torch.from_numpy(w.logits).to(dev)
         masks = None if w.masks is None else torch.from_numpy(w.masks.view(np.int32)).to(dev)
         hist, hl = torch.from_numpy(w.history).to(dev), torch.from_numpy(w.history_len).to(dev)

@@ -1,7 +1,7 @@
 """The bulk-copy kernel (k_ring) and the cluster kernel (k_cluster) against the oracle on the inputs that stress them.
 
-Calls of many rows take k_ring when they have no mask, and always when k_cap exceeds 512 (then also under a mask);
-small batches with k_cap up to 128 take k_cluster.  The cases below pick k_cap and masks accordingly and say which
+Calls of many rows take k_ring when they have no mask, and always when k_cap exceeds 512 (then also under a mask); under
+masks they take k_rows with k_cap up to 128 and k_select with 129 to 512.  Small batches with k_cap up to 128 take k_cluster.  The cases below pick k_cap and masks accordingly and say which
 kernel a small batch is meant for (run_rows' cluster_rows).  Everything goes through the C ABI; candidates must be
 bit-exact and tokens equal (or on a CDF boundary within 1e-6), as in test_parity_gpu.py.
 """
@@ -43,7 +43,7 @@ def test_ragged_vocabularies_masked_and_unmasked(dev, oracle, n, bf16):
     check_against_oracle(oracle, w2, *run_rows(w2, dev, max_history=64, cluster_rows=6))   # six clusters
     w3 = wl.Workload("ragged_masked_k64", logits, p, masks, hist, hl, bf16=bf16, k_cap=64)
     check_against_oracle(oracle, w3, *run_rows(w3, dev, max_history=64, cluster_rows=6))   # six clusters, under the masks
-    check_against_oracle(oracle, w3, *run_rows(w3, dev, max_history=64, cluster_rows=0))   # k_select
+    check_against_oracle(oracle, w3, *run_rows(w3, dev, max_history=64, cluster_rows=0))   # k_rows
 
 
 def test_equal_values_take_the_careful_walk(dev, oracle):
@@ -69,7 +69,7 @@ def test_equal_values_take_the_careful_walk(dev, oracle):
             check_against_oracle(oracle, w, tokens, cands)
             if temperature == 0.0:
                 assert tokens[1] == 0  # no history: the first of all the equal values
-    # the same rows under masks go through k_select: a greedy row whose work list overflows takes its careful walk
+    # the same rows under masks go through k_rows: a greedy row flags every cell, more than its buffer holds
     masks = np.stack([wl.run_mask(wl.rng(3 + r), n, 0.7, 20) for r in range(6)])
     p = make_params(6, temperature=0.0, repetition=1.2, presence=0.4, frequency=0.01)
     w = wl.Workload("equal_masked", x, p, masks, hist, hl)
@@ -219,3 +219,29 @@ def test_one_verification_window_of_four_columns(dev, oracle):
     et, ea = oracle.verify_window(sw.logits, sw.draft[0], sw.params, masks=masks, hist=hist[0])
     assert np.array_equal(toks.cpu().numpy(), et) and acc.item() == ea
     s.close()
+
+
+@pytest.mark.parametrize("k_cap", [129, 256, 384, 385, 512])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_masked_batches_of_middling_k(dev, oracle, k_cap, bf16):
+    """k_cap 129 to 512 under masks: whole rows through k_select.  Equal values that overflow its work list and its buffer,
+    histories of the best ids with repeats, greedy rows, sparse and full masks; rows on and off 16-byte boundaries."""
+    g = wl.rng(k_cap + bf16)
+    rows = 7
+    for n in (40_000, 40_003):  # (rows lie side by side: with the odd length they start anywhere)
+        x = wl.gaussian_logits(g, rows, n, 2.5)
+        x[1] = 1.25
+        x[2] = np.repeat(np.arange(n // 64 + 1, dtype=np.float32), 64)[:n] / 8
+        x[3] = np.linspace(-8, 8, n, dtype=np.float32)
+        if bf16:
+            x = wl.bf16_bits_to_f32(wl.f32_to_bf16_bits(x))
+        masks = np.stack([wl.random_mask(g, n, d) for d in (1.0, 0.9, 1.0, 0.6, 0.01, 0.2, 0.5)])
+        hist = g.integers(-2, n + 2, size=(rows, 900), dtype=np.int32)
+        hist[0, :400] = np.argsort(-x[0])[:400]
+        hist[5, :400] = np.repeat(np.argsort(-x[5])[:100], 4)
+        p = make_params(rows, temperature=0.9, top_k=0, top_p=0.97, min_p=0.001, repetition=1.1, presence=0.3, frequency=0.2, seed=k_cap)
+        p["temperature"][6] = 0.0
+        p["frequency"][5] = -0.1
+        logits = wl.f32_to_bf16_bits(x) if bf16 else x
+        w = wl.Workload("middling", logits, p, masks, hist, np.full(rows, 900, np.int32), bf16=bf16, k_cap=k_cap)
+        check_against_oracle(oracle, w, *run_rows(w, dev, max_history=900))

@@ -327,15 +327,23 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
             const uint32_t f = pen_pos(ids[u]);
             if (f != 0xffffffffu && ((atomicOr(&hb[f >> 5], 1u << (f & 31)) >> (f & 31)) & 1u)) again |= 1u << u;
         }
-        if (!__any_sync(kFull, again != 0u) || p.frequency == 0.0f) continue;
-#pragma unroll 1
-        for (uint32_t q = again; q; q &= q - 1u) {
-            const int u0 = __ffs(q) - 1;
-            int32_t id = ids[0];
+        if (p.frequency == 0.0f || !__any_sync(kFull, again != 0u)) continue;
+        // (one reservation per warp: a history that repeats itself has more of these than others)
+        const uint32_t mine_n = (uint32_t) __popc(again);
+        uint32_t upto = mine_n;
 #pragma unroll
-            for (int u = 1; u < HB; ++u) id = u == u0 ? ids[u] : id;
-            const uint32_t at = atomicAdd(&sh.n_own, 1u);
-            if (at < (uint32_t) kRowsDups) dups[at] = pen_pos(id);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, upto, o);
+            if (lane >= o) upto += t;
+        }
+        uint32_t at = 0u;
+        if (lane == 31) at = atomicAdd(&sh.n_own, upto);
+        at = __shfl_sync(kFull, at, 31) + upto - mine_n;
+#pragma unroll
+        for (int u = 0; u < HB; ++u) {
+            if (!((again >> u) & 1u)) continue;
+            if (at < (uint32_t) kRowsDups) dups[at] = pen_pos(ids[u]);
+            ++at;
         }
     }
     if (rank == 0 && tid == NT - 1) {  // what the draw needs (column c of a window draws with counter + c, src/engine.cu:756)
@@ -404,11 +412,8 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
             tcnt[slot] = short_list ? 1u : 0u;
         }
         __syncthreads();
-        const int n_walk = short_list ? (int) n_dup : n_pen;
-#pragma unroll 1
-        for (int t = tid; t < n_walk; t += NT) {
-            const uint32_t o = short_list ? dups[t] : pen_pos(pen_id(t));
-            if (o == 0xffffffffu) continue;
+        auto count = [&](uint32_t o) {
+            if (o == 0xffffffffu) return;
             uint32_t q = (o * 2654435761u) >> kTShift;
             for (uint32_t kx = tkey[q]; kx != kNoKey; kx = tkey[q]) {  // at most NT keys in 2 NT slots
                 if (kx == o) {
@@ -417,6 +422,18 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
                 }
                 q = (q + 1u) & (TS - 1);
             }
+        };
+        const int n_walk = short_list ? (int) n_dup : n_pen;
+#pragma unroll 1
+        for (int t0 = tid; t0 < n_walk; t0 += 4 * NT) {  // (the ids of a round are requested together)
+            uint32_t o[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int t = t0 + u * NT;
+                o[u] = t >= n_walk ? 0xffffffffu : (short_list ? dups[t] : pen_pos(pen_id(t)));
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) count(o[u]);
         }
         __syncthreads();
         float n = 1.0f;

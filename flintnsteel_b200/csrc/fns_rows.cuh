@@ -44,8 +44,6 @@ struct RowsShared {
     fns_b200_params p;                   // the row's parameters
     uint32_t n_hl;                       // cursor of the list of history ids that need their occurrences
     uint32_t count[kRowsMaxCtas];        // how many keys every CTA sent to CTA 0
-    uint32_t local_bound[kRowsMaxCtas];  // second chance: the bound that each CTA could make of its own threads' maxima
-    __align__(16) uint32_t wit[256];     // the row's witnesses (every CTA gets a copy)
     uint32_t hl_pos[kRowsThreads];       // the list: positions f
     float hl_raw[kRowsThreads];          // ... and logits
     __align__(16) uint32_t lut[64];      // fill_or_masks
@@ -113,7 +111,8 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
     uint64_t * sorted = sel + a.k_cap;                                      // [k_cap]
     double * pj = reinterpret_cast<double *>(sorted + a.k_cap);             // [k_cap]
     double * acc = pj + a.k_cap;                                            // [k_cap]
-    uint32_t * eff = reinterpret_cast<uint32_t *>(acc + a.k_cap);           // [eff_words] under a mask: bit f is allowed and in a whole vector
+    uint32_t * wit = reinterpret_cast<uint32_t *>(acc + a.k_cap);           // [C * NT] the row's witnesses (every CTA gets a copy)
+    uint32_t * eff = wit + C * NT;                                          // [eff_words] under a mask: bit f is allowed and in a whole vector
     uint32_t * hb = eff + (listed ? eff_words : 0);                         // [eff_words] with a history: bit f is a history id
     uint32_t * tkey = hb + (a.own_cap > 0 ? eff_words : 0);                 // [TS]
     uint32_t * tcnt = tkey + TS;                                            // [TS]
@@ -388,7 +387,7 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
         uint32_t w = wt;
         for (int o = 1; o < C; o <<= 1) w = max(w, __shfl_xor_sync(kFull, w, o));
         // lane j of a group of C lanes sends the group's maximum to CTA j
-        cluster.map_shared_rank(&rs, tid & (C - 1))->wit[rank * (NT >> lg_c) + (tid >> lg_c)] = w;
+        cluster.map_shared_rank(wit, tid & (C - 1))[rank * (NT >> lg_c) + (tid >> lg_c)] = w;
     }
     if (C > 1) cluster.sync();
     else __syncthreads();
@@ -444,6 +443,55 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
     };
     auto is_hist = [&](uint32_t f) -> bool { return (hb[f >> 5] >> (f & 31)) & 1u; };
 
+    // What a thread's cells without a history id say for certain: the largest of their maxima, or what the heaviest penalty of
+    // the row leaves of the largest of its other cells (penalties that only lower keep the order, so whatever held that
+    // maximum does not end below it) - from the cells' 16-bit maxima, cut the other way where they are negative.  About
+    // 3 us of a block, which is why only a row takes it whose history shows among the best.
+    auto clean_witness = [&]() -> uint32_t {
+        uint32_t * mark = vlist;                                 // [2 NT] bit c: cell c of the thread holds a history id
+        uint16_t * seg_at = reinterpret_cast<uint16_t *>(lbuf);  // the places of the listed segments
+        static_assert(kWarps * kWarpList >= 2 * NT && kRowsBuf * 4 >= kRowsMaxCells * NV * kWarps, "room for the marks");
+        __syncthreads();
+        mark[tid] = mark[NT + tid] = 0u;
+        if (listed)
+            for (int i = tid; i < n_list; i += NT) seg_at[entry(i) & 0x7fffu] = (uint16_t) i;
+        __syncthreads();
+#pragma unroll 4
+        for (int j = tid; j < n_pen; j += NT) {
+            const uint32_t f = pen_pos(pen_id(j));
+            const int e = (int) f - h;  // the element's number in the whole vectors
+            if (f == 0xffffffffu || e < 0 || e >= nv * VEC || (listed && !((eff[f >> 5] >> (f & 31)) & 1u))) continue;
+            const int seg = e / (32 * VEC), at = listed ? (int) seg_at[seg] : seg;  // (an allowed id: its segment is on the list)
+            const int c = at / (NV * kWarps);
+            atomicOr(&mark[(c >> 5) * NT + (at % kWarps) * 32 + (e / VEC) % 32], 1u << (c & 31));
+        }
+        __syncthreads();
+        const uint32_t q_lo = mark[tid], q_hi = mark[NT + tid];
+        float clean = -INFINITY, other = -INFINITY;
+#pragma unroll 2
+        for (int c = 0; c < n_cells; ++c) {
+            const float m = __uint_as_float((uint32_t) cmax[c * NT + tid] << 16);
+            if (((c < 32 ? q_lo >> c : q_hi >> (c - 32)) & 1u) == 0u) clean = fmaxf(clean, m);
+            else other = fmaxf(other, m);
+        }
+        auto down = [](float m) -> float { return __uint_as_float(__float_as_uint(m) | ((int) __float_as_uint(m) < 0 ? 0xffffu : 0u)); };
+        float w = clean > other ? tmax : down(clean);  // (NaN for -inf: never wins)
+        if (!(clean > other) && lowering) w = fmaxf(w, penalised(down(other), p.frequency != 0.0f ? (float) (1u + sh.n_own) : 1.0f));
+        __syncthreads();  // (mark and lbuf are used again)
+        return w >= -FLT_MAX ? order_word(w) : 0u;
+    };
+    int n_wit = NT;  // witnesses of groups, or (C * NT) of threads
+    auto send_all = [&](uint32_t w) {  // a thread's witness to every CTA
+        if (C > 1) cluster.sync();     // (every CTA has read the ones before)
+        else __syncthreads();
+        for (int r = 0; r < C; ++r) cluster.map_shared_rank(wit, r)[rank * NT + tid] = w;
+        n_wit = C * NT;
+        if (C > 1) cluster.sync();
+        else __syncthreads();
+    };
+    // More history ids than six for ten cells leave few cells without one: a lower bound is tried first.
+    bool crowded = 5ll * n_pen * (VEC * NV) > 3ll * a.vocab;
+    bool sure = n_pen == 0;
     // From here on once, and again with a lower bound if history ids took too many candidates away.
     int witnesses = n_pen > 0 ? min(k + (k >> 2) + 8, 256) : k;  // how many must reach the bound
     float thr_v;
@@ -452,15 +500,12 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
     int n_all;
     const int region = kRowsGather >> lg_c;  // what a CTA may send to CTA 0 (k_cap at least)
     for (;;) {
-        // 5. The bound.
+        // 5. The bound.  (Too few groups saw anything, as under a mask that leaves little: every thread speaks for itself.)
         int reach;
-        uint32_t bound = block_reach<NT>([&](int i) { return rs.wit[i]; }, NT, witnesses, 4, sh.sc, sh.ends, &reach);
-        if (C > 1 && bound == 0u) {  // too few groups saw anything: the largest bound that a CTA can make alone
-            __syncthreads();
-            const uint32_t mine = block_reach<NT>([&](int) { return wt; }, NT, witnesses, 4, sh.sc, sh.ends, &reach);
-            if (tid < C) cluster.map_shared_rank(&rs, tid)->local_bound[rank] = mine;
-            cluster.sync();
-            for (int r = 0; r < C; ++r) bound = max(bound, rs.local_bound[r]);
+        uint32_t bound = block_reach<NT>([&](int i) { return wit[i]; }, n_wit, witnesses, 4, sh.sc, sh.ends, &reach);
+        if (C > 1 && bound == 0u && n_wit == NT) {
+            send_all(wt);
+            bound = block_reach<NT>([&](int i) { return wit[i]; }, n_wit, min(witnesses, k), 4, sh.sc, sh.ends, &reach);
         }
         const bool bounded = bound != 0u;
         thr_v = bounded ? word_value(bound) + 0.0f : -FLT_MAX;  // (-0.0 -> +0.0: one key pattern for both)
@@ -590,16 +635,26 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
             }
         }
         __syncthreads();
-        // Every history id, once each (penalties that can raise a value): the thread that takes the id's bit away owns it.
-        auto every_history_id = [&](auto take) {
+        // The history ids that are on the list, whose occurrences are counted now.
+        auto listed_history_ids = [&](uint32_t n_hl) {
+            const bool live = (uint32_t) tid < n_hl;
+            const uint32_t f = live ? rs.hl_pos[tid] : 0u;
+            const float cnt = occurrences(live, f), v = live ? penalised(rs.hl_raw[tid], cnt) : -INFINITY;
+            offer(v >= thr_v && is_finite(v) ? make_key(v, id0 + f) : 0ull);
+            __syncthreads();
+        };
+        // Every history id, once each (penalties that can raise a value, or more of them than the list holds).
+        auto every_history_id = [&]() {  // (the thread that takes an id's bit away owns it)
 #pragma unroll 1
             for (int j0 = 0; j0 < n_pen; j0 += NT) {
                 const uint32_t f = j0 + tid < n_pen ? pen_pos(pen_id(j0 + tid)) : 0xffffffffu;
                 bool live = f != 0xffffffffu && allowed(f);
                 if (live) live = (atomicAnd(&hb[f >> 5], ~(1u << (f & 31))) >> (f & 31)) & 1u;
+                const float raw = live ? to_float(x[f]) : 0.0f;
+                if (lowering) live = live && penalised(raw, 1.0f) >= thr_v;
                 const float cnt = p.frequency != 0.0f ? occurrences(live, f) : 1.0f;
-                const float v = live ? penalised(to_float(x[f]), cnt) : -INFINITY;
-                take(v >= thr_v && is_finite(v) ? make_key(v, id0 + f) : 0ull);
+                const float v = live ? penalised(raw, cnt) : -INFINITY;
+                offer(v >= thr_v && is_finite(v) ? make_key(v, id0 + f) : 0ull);
             }
             __syncthreads();
 #pragma unroll 1
@@ -612,76 +667,84 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
         if (n_pen > 0) {
             if (lowering) {
                 const uint32_t n_hl = rs.n_hl;
-                if (n_hl > 0u && n_hl <= (uint32_t) NT) {  // uniform
-                    const bool live = (uint32_t) tid < n_hl;
-                    const uint32_t f = live ? rs.hl_pos[tid] : 0u;
-                    const float cnt = occurrences(live, f), v = live ? penalised(rs.hl_raw[tid], cnt) : -INFINITY;
-                    offer(v >= thr_v && is_finite(v) ? make_key(v, id0 + f) : 0ull);
-                    __syncthreads();
-                }
+                // (too few even if all of them stay: their occurrences can wait for the next bound)
+                const bool enough = C > 1 || sure || !bounded || (int) (sh.n_cand + n_hl) >= k;
+                if (n_hl > 0u && n_hl <= (uint32_t) NT && enough) listed_history_ids(n_hl);  // uniform
             } else {
-                every_history_id(offer);
+                every_history_id();
             }
         }
         int n_loc = (int) sh.n_cand;
         keys = lbuf;
-        if (n_loc > kRowsBuf || sh.n_vl != 0u || rs.n_hl > (uint32_t) NT) {  // uniform in the CTA
-            // Many equal values (or history ids): everything is offered again from an empty buffer, one element per thread
-            // and round, with a vote after every round on whether to compact, which also raises the bar.
-            __syncthreads();
-            if (tid == 0) sh.n_cand = 0u;
-            __syncthreads();
-            auto settle = [&](uint64_t key) {
-                bool lost = key != 0ull && key >= thr_key && !push(key, lbuf, sh, kRowsBuf);
-                while (__syncthreads_or(lost || *(volatile uint32_t *) &sh.n_cand >= (uint32_t) kRowsBuf / 2)) {
-                    compact<NT>(lbuf, sel, k, kRowsBuf, sh);
-                    const uint64_t tk = sh.thr_key;
-                    if (tk > thr_key) {
-                        thr_key = tk;
-                        thr_v = key_floor_value(tk);
-                    }
-                    if (lost && (key < thr_key || push(key, lbuf, sh, kRowsBuf))) lost = false;
-                    if (!__syncthreads_or(lost)) break;
+        if (__builtin_expect(n_loc > kRowsBuf || sh.n_vl != 0u || rs.n_hl > (uint32_t) NT, 0)) {  // uniform in the CTA
+            // More than the lists or the buffer hold.  The k-th best of a full buffer is a bound that k candidates reach: with it
+            // everything is offered again, a cell per thread and round, until it fits.  It is a whole key, so that equal values
+            // are cut by their ids, and every time it rises past all but k of the buffer.  (An element per thread between block
+            // votes, as k_cluster does it, took 0.4 to 1.7 ms for a batch of rows whose best ids are in the history.)
+            for (;;) {
+                __syncthreads();
+                if (n_loc > kRowsBuf) {
+                    thr_key = block_kth_key<NT>(lbuf, kRowsBuf, k, sh.sc);
+                    thr_v = key_floor_value(thr_key);
                 }
-            };
-            auto settle_element = [&](bool ok, float raw, uint32_t f) {
-                if (n_pen > 0) {
-                    bool live = ok && is_hist(f);
-                    if (!lowering && live) ok = live = false;
-                    float v = raw;
-                    if (live) v = penalised(raw, 1.0f);
-                    if (p.frequency != 0.0f && lowering) {
-                        live = live && v >= thr_v;
-                        const float cnt = occurrences(live, f);
-                        if (live) v = penalised(raw, cnt);
-                    }
-                    raw = v;
+                if (tid == 0) {
+                    sh.n_cand = 0u;
+                    rs.n_hl = 0u;
                 }
-                settle(ok && raw >= thr_v && is_finite(raw) ? make_key(raw, id0 + f) : 0ull);
-            };
-            settle_element(rag_ok && rag_x >= thr_v && rag_x <= FLT_MAX, rag_x, (uint32_t) rag_f);
+                __syncthreads();
+                const float cut = __uint_as_float(__float_as_uint(thr_v) & 0xffff0000u);
 #pragma unroll 1
-            for (int v0 = 0; v0 < nv; v0 += NT) {
-                const uint32_t bits = v0 + tid < nv ? vector_bits(v0 + tid) : 0u;
-                float xs[VEC];
-                if (bits) load_vec<T, VEC>(reinterpret_cast<const T *>(vector_at(v0 + tid)), xs);
-#pragma unroll 1
-                for (int j = 0; j < VEC; ++j) {
-                    float xj = xs[0];
+                for (int c = -1; c < n_cells; ++c) {  // (-1: the elements outside whole vectors)
+                    const bool take = c < 0 ? rag_ok : tmax >= thr_v && __uint_as_float((uint32_t) cmax[c * NT + tid] << 16) >= cut;
+                    const bool full = __shfl_sync(kFull, *(volatile uint32_t *) &sh.n_cand, 0) > (uint32_t) kRowsBuf;
+                    if (full || !__any_sync(kFull, take)) continue;
+                    uint4 r[NV];
+                    uint32_t bits[NV];
 #pragma unroll
-                    for (int e = 1; e < VEC; ++e) xj = e == j ? xs[e] : xj;
-                    settle_element(((bits >> j) & 1u) && xj >= thr_v && xj <= FLT_MAX, xj, (uint32_t) (h + (v0 + tid) * VEC + j));
+                    for (int u = 0; u < NV; ++u) {
+                        const int v = c < 0 ? 0 : (int) (entry((c * NV + u) * kWarps + warp) & 0x7fffu) * 32 + lane;
+                        bits[u] = take && c >= 0 ? vector_bits(v) : 0u;
+                        r[u] = make_uint4(0u, 0u, 0u, 0u);
+                        load_if(r[u], vector_at(v), bits[u]);
+                    }
+#pragma unroll 1
+                    for (int u = 0; u < NV; ++u) {
+                        float xs[VEC];
+                        raw_values<T, VEC>(u == 0 ? r[0] : (u == 1 ? r[1] : (u == 2 ? r[2] : r[3])), xs);
+                        const uint32_t b = u == 0 ? bits[0] : (u == 1 ? bits[1] : (u == 2 ? bits[2] : bits[3]));
+                        const int f_v = c < 0 ? 0 : h + ((int) (entry((c * NV + u) * kWarps + warp) & 0x7fffu) * 32 + lane) * VEC;
+#pragma unroll 1
+                        for (int j = 0; j < VEC; ++j) {
+                            float raw = xs[0];
+#pragma unroll
+                            for (int e = 1; e < VEC; ++e) raw = e == j ? xs[e] : raw;
+                            bool ok = (b >> j) & 1u;
+                            uint32_t f = (uint32_t) (f_v + j);
+                            if (c < 0 && u == 0 && j == 0) {
+                                ok = take;
+                                raw = rag_x;
+                                f = (uint32_t) rag_f;
+                            }
+                            ok = ok && raw >= thr_v && raw <= FLT_MAX;
+                            if (!__any_sync(kFull, ok)) continue;
+                            offer(!ok ? 0ull : (n_pen > 0 && is_hist(f) ? history_key(raw, f) : make_key(raw, id0 + f)));
+                        }
+                    }
                 }
+                __syncthreads();
+                if (n_pen > 0) {
+                    const uint32_t n_hl = rs.n_hl;  // uniform
+                    if (!lowering || n_hl > (uint32_t) NT) {
+                        every_history_id();
+                    } else if (n_hl > 0u) {
+                        listed_history_ids(n_hl);
+                    }
+                }
+                n_loc = (int) sh.n_cand;
+                if (n_loc <= kRowsBuf) break;  // uniform in the CTA
             }
-            if (!lowering) every_history_id(settle);
-            __syncthreads();
-            n_loc = (int) min(sh.n_cand, (uint32_t) kRowsBuf);
         }
-        if (C > 1 && n_loc > region) {  // only this CTA's best k can matter
-            const uint64_t tau = block_kth_key<NT>(lbuf, n_loc, k, sh.sc);
-            n_loc = block_take<NT>(lbuf, n_loc, k, tau, sel, sh.sc);
-            keys = sel;
-        }
+        if (C > 1 && n_loc > region) keys = best_keys<NT>(lbuf, &n_loc, k, a.k_cap - k, sorted, a.k_cap, sel, sh);  // only this CTA's best k can matter
         n_all = n_loc;
         if (C > 1) {
             if (tid < C) cluster.map_shared_rank(&rs, tid)->count[rank] = (uint32_t) n_loc;
@@ -691,16 +754,17 @@ __global__ void __launch_bounds__(kRowsThreads, 3) k_rows(const SelectArgs a) {
             n_all = 0;
             for (int q = 0; q < C; ++q) n_all += (int) rs.count[q];
         }
-        if (n_pen == 0 || n_all >= k || !bounded) break;  // (the same in every CTA of the cluster)
-        if (C > 1) cluster.sync();  // (every CTA has read the counts)
-        else __syncthreads();
+        if (sure || n_all >= k || !bounded) break;  // (the same in every CTA of the cluster)
+        // History ids took too many away: once more with a bound that they have no part in, or with a lower one.
+        send_all(crowded ? wt : clean_witness());
+        sure = !crowded;
+        witnesses = crowded ? 2 * witnesses : k;  // (more than there are: no bound at all)
+        crowded = false;
         if (tid == 0) {
             sh.n_cand = 0u;
-            sh.thr_key = 0ull;
             sh.n_vl = 0u;
             rs.n_hl = 0u;
         }
-        witnesses = witnesses < 256 ? min(2 * witnesses, 256) : 257;  // (257: no bound at all)
         __syncthreads();
     }
     if (C > 1) {

@@ -564,19 +564,17 @@ __device__ __forceinline__ void rank_draw(const uint64_t * buf, int n, int k, ui
     draw_warp(sorted, nk, pj, acc, qj, u01, p, out_token);
 }
 
-// What rank_draw would take long for: cuts keys[0 .. n) to little more than the best k by their order words, in `to` (room
-// for kRankSelectMax keys, not keys itself), or to the best k in sel when equal values leave too many.  Returns where they
-// are now and sets *n.  The cut costs about what ranking 192 keys in 256 threads does; 400 keys take four times that.
-// All NT threads; block synchronised on entry and exit.
-constexpr int kCutMin = 192;
+// The best k of keys[0 .. n), and at most `slack` others unless equal values leave no choice, found by their order words and
+// moved to `to` (room for that many); the best k alone to sel when more than `room` reach that word.  Returns where they are
+// now and sets *n.  keys, to and sel are different places.  All NT threads; block synchronised on entry and exit; n > k.
 template <int NT>
-__device__ __forceinline__ uint64_t * cut_keys(uint64_t * keys, int * n, int k, uint64_t * to, uint64_t * sel, SelectShared & sh) {
+__device__ __forceinline__ uint64_t * best_keys(uint64_t * keys, int * n, int k, int slack, uint64_t * to, int room, uint64_t * sel,
+                                                SelectShared & sh) {
     SelectScratch & sc = sh.sc;
     const int have = *n;
-    if (have <= k || have <= kCutMin) return keys;
     int reach;
-    const uint32_t bar = block_reach<NT>([&](int i) { return (uint32_t) (keys[i] >> 32); }, have, k, k >> 3, sc, sh.ends, &reach);
-    if (reach > kRankSelectMax) {
+    const uint32_t bar = block_reach<NT>([&](int i) { return (uint32_t) (keys[i] >> 32); }, have, k, slack, sc, sh.ends, &reach);
+    if (reach > room) {
         __syncthreads();
         const uint64_t tau = block_kth_key<NT>(keys, have, k, sc);
         *n = block_take<NT>(keys, have, k, tau, sel, sc);
@@ -591,6 +589,15 @@ __device__ __forceinline__ uint64_t * cut_keys(uint64_t * keys, int * n, int k, 
     __syncthreads();
     *n = reach;
     return to;
+}
+
+// What rank_draw would take long for: cuts keys[0 .. n) to little more than the best k.  The cut costs about what ranking 192
+// keys in 256 threads does; 400 keys take four times that.  `to` has room for kRankSelectMax keys.
+constexpr int kCutMin = 192;
+template <int NT>
+__device__ __forceinline__ uint64_t * cut_keys(uint64_t * keys, int * n, int k, uint64_t * to, uint64_t * sel, SelectShared & sh) {
+    if (*n <= k || *n <= kCutMin) return keys;
+    return best_keys<NT>(keys, n, k, k >> 3, to, kRankSelectMax, sel, sh);
 }
 
 // Largest float of the allowed, finite elements of one vector (-inf if none).  NaN never wins an fmaxf and
@@ -1829,7 +1836,7 @@ bool make_rows_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, 
         pl.own_cap = hist_bound;                                // (more than 0: the kernel has a bit set of history ids)
         pl.seg_cap = round_up(pl.slice_len / 32 + vec + 2, 4);  // words of a bit set: the slice and, all 0, one more segment
         pl.list_cap = masked ? pl.n_stages * kRowsCell * (kRowsThreads / 32) : 0;  // places: whole cells
-        pl.smem_select = ((sizeof(RowsShared) + 15) & ~(size_t) 15) + (size_t) (kRowsBuf + kRowsGather) * 8 + (size_t) k_cap * 8 * 4 +
+        pl.smem_select = ((sizeof(RowsShared) + 15) & ~(size_t) 15) + (size_t) (kRowsBuf + kRowsGather) * 8 + (size_t) k_cap * 8 * 4 + (size_t) c * kRowsThreads * 4 +
                          (size_t) pl.seg_cap * 4 * ((masked ? 1 : 0) + (hist_bound > 0 ? 1 : 0)) + (size_t) kRowsThreads * 2 * 8 +
                          (size_t) (kRowsThreads / 32) * kWarpList * 4 + (hist_bound > 0 ? (size_t) kRowsDups * 4 : 0) +
                          (size_t) pl.n_stages * kRowsThreads * 2 + (size_t) pl.list_cap * 2;

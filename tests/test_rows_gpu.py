@@ -1,10 +1,10 @@
-"""The batch kernel (k_rows: a row cut over a cluster of 1, 2 or 4 CTAs, any alignment) against the oracle, at the sizes where
-it can go wrong, and sparse masks through both cluster kernels."""
+"""The batch kernel (k_rows: a row cut over a cluster of 1, 2, 4 or 8 CTAs, any alignment) against the oracle, at the sizes
+where it can go wrong, and what a batch may cost when its histories or masks are not noise."""
 import numpy as np
 import pytest
 
 from flintnsteel_b200 import workloads as wl
-from flintnsteel_b200.sampler import Sampler, make_params, params_to_device
+from flintnsteel_b200.sampler import BF16, F32, Sampler, cands_tensor, cands_to_numpy, make_params, params_to_device
 
 from .test_parity_gpu import check_against_oracle, dev, run_rows, upload  # noqa: F401  (dev is a fixture)
 
@@ -32,6 +32,14 @@ def batch(g, rows, n, bf16=False, hist=64, top_hist=False, fractions=(1.0, 0.5, 
     return wl.Workload("rows", logits, p, masks, np.ascontiguousarray(h), np.full(rows, hist, np.int32), bf16=bf16)
 
 
+def plan_slices(w, max_history):
+    s = Sampler(0, max_rows=w.rows, max_vocab=w.vocab, k_cap=w.k_cap, max_history=max_history)
+    s.set_cluster_rows(0)
+    slices = s.plan(BF16 if w.bf16 else F32, w.vocab, w.rows, max_history)["slices"]
+    s.close()
+    return slices
+
+
 @pytest.mark.parametrize("bf16", [False, True])
 @pytest.mark.parametrize("n", [1, 3, 7, 255, 256, 257, 4095, 32_768, 65_537, 131_071])
 @pytest.mark.parametrize("rows", [5, 37])
@@ -46,13 +54,14 @@ def test_rows_of_any_length_packed_side_by_side(dev, oracle, n, rows, bf16):
 
 @pytest.mark.parametrize("rows", [16, 64, 150])
 def test_slices_of_a_full_vocabulary(dev, oracle, rows):
-    """4, 4 and 1 CTAs per row; more history ids among the best than the bound allows for, so that it is lowered; allowed
+    """4, 4 and 2 CTAs per row; more history ids among the best than the bound allows for, so that it is lowered; allowed
     ids in one slice only; few allowed ids, so that there is no bound."""
     g = wl.rng(rows)
     n = wl.V_QWEN
     w = batch(g, rows, n, hist=400, top_hist=True, fractions=(1.0, 0.3, 0.01, 0.003, 0.0005))
     w.masks[1::7] = 0
     w.masks[1::7, 100:170] = 0xFFFFFFFF
+    assert plan_slices(w, 400) == {16: 4, 64: 4, 150: 2}[rows]
     check_against_oracle(oracle, w, *run_rows(w, dev, max_history=400, cluster_rows=0))
     check_against_oracle(oracle, w, *run_rows(w, dev, k_cap=128, max_history=400, cluster_rows=0), k_cap=128)
 
@@ -88,6 +97,94 @@ def test_crowds_of_equal_values(dev, oracle):
     p["frequency"][7] = -0.5
     w = wl.Workload("crowds", x, p, masks, hist, np.full(8, 600, np.int32))
     check_against_oracle(oracle, w, *run_rows(w, dev, max_history=600, cluster_rows=0))
+
+
+def hot_history(g, x, masks, hist, hot, spread):
+    """hist ids per row of which the first ones are the row's `hot` best allowed ids, the rest drawn from the vocabulary; `spread`
+    > 0: drawn again with repeats from that many different ones."""
+    rows, n = x.shape
+    h = g.integers(0, n, size=(rows, hist), dtype=np.int32)
+    for r in range(rows):
+        xr = x[r].copy()
+        if masks is not None:
+            xr[~wl.mask_allows(masks[r], np.arange(n))] = -np.inf
+        best = np.argsort(-xr, kind="stable")[:min(hot, hist)]
+        h[r, :best.size] = best
+        if spread:
+            h[r] = g.choice(h[r, :spread], size=hist)
+    return h
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("hot, hist, spread", [(100, 300, 0), (400, 2048, 0), (2048, 2048, 0), (200, 2048, 600), (300, 16_384, 0)])
+@pytest.mark.parametrize("n, rows", [(151_936, 7), (32_003, 37)])
+def test_the_best_ids_are_in_the_history(dev, oracle, n, rows, hot, hist, spread, bf16):
+    """Rows whose best ids are penalised, once each and with repeats, few and so many that history ids lie in every cell; cut
+    rows, whole rows and rows off a 16-byte boundary; with and without a frequency penalty, strong and raising ones."""
+    g = wl.rng(hot + hist + spread + n + bf16)
+    x = wl.gaussian_logits(g, rows, n, 2.5)
+    if bf16:
+        x = wl.bf16_bits_to_f32(wl.f32_to_bf16_bits(x))
+    masks = np.stack([wl.run_mask(g, n, f) for f in (1.0, 0.5, 0.05, 0.01, 0.004)[:rows] * -(-rows // 5)])[:rows]
+    h = hot_history(g, x, masks, hist, hot, spread)
+    p = make_params(rows, temperature=0.8, top_p=0.95, repetition=1.1, presence=0.5, frequency=0.3, seed=3)
+    p["top_k"] = g.choice(np.array([0, 1, 20, 64], np.int32), size=rows)
+    p["repetition"][1::5], p["presence"][1::5], p["frequency"][1::5] = 2.0, 0.0, 0.0
+    p["repetition"][2::5], p["presence"][2::5], p["frequency"][2::5] = 1.0, 0.0, 1.0
+    p["repetition"][3::5] = 0.8
+    p["frequency"][4::5] = 0.0
+    w = wl.Workload("hot", wl.f32_to_bf16_bits(x) if bf16 else x, p, masks, h, np.full(rows, hist, np.int32), bf16=bf16)
+    check_against_oracle(oracle, w, *run_rows(w, dev, max_history=hist, cluster_rows=0))
+
+
+def test_whole_rows_of_more_than_32_cells(dev, oracle):
+    """223 rows and more are not cut; the best ids and the history lie behind cell 32 of 38 (element 131,072 on)."""
+    g = wl.rng(38)
+    rows, n = 224, wl.V_QWEN
+    x = wl.gaussian_logits(g, rows, n, 2.5)
+    x[:, 131_072:] += 4.0
+    masks = np.full((rows, n // 32), 0xFFFFFFFF, np.uint32)
+    masks[::3] = wl.random_mask(g, n, 0.7)
+    w = wl.Workload("deep", x, make_params(rows, temperature=0.8, top_p=0.95, top_k=50, repetition=1.2, presence=0.3, frequency=0.2, seed=2),
+                    masks, None, None)
+    w.params["temperature"][::4] = 0.0
+    w.history = g.integers(131_000, n, size=(rows, 300), dtype=np.int32)
+    w.history[1::2, :40] = np.argsort(-x[1::2], axis=1)[:, :40]
+    w.history_len = np.full(rows, 300, np.int32)
+    assert plan_slices(w, 300) == 1
+    check_against_oracle(oracle, w, *run_rows(w, dev, max_history=300, cluster_rows=0))
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows", [6, 40])
+def test_a_shard_with_a_history_of_global_ids(dev, oracle, rows, bf16):
+    """select_rows with id_base: masks, a history of ids inside and outside the shard, k_cap 64 and 128."""
+    g = wl.rng(rows + bf16)
+    base, n = 65_536, 40_001
+    x = wl.gaussian_logits(g, rows, n, 2.5)
+    if bf16:
+        x = wl.bf16_bits_to_f32(wl.f32_to_bf16_bits(x))
+    masks = np.stack([wl.run_mask(g, n, (1.0, 0.2, 0.01)[r % 3]) for r in range(rows)])
+    h = g.integers(0, 2 * base, size=(rows, 500), dtype=np.int32)
+    h[:, :60] = base + np.argsort(-x, axis=1)[:, :60]
+    h[:, 60:80] = h[:, :20]
+    p = make_params(rows, temperature=0.8, top_k=0, repetition=1.2, presence=0.3, frequency=0.2)
+    lg = torch.from_numpy(wl.f32_to_bf16_bits(x).view(np.int16)).to(dev).view(torch.bfloat16) if bf16 else torch.from_numpy(x).to(dev)
+    for k in (64, 128):
+        s = Sampler(0, max_rows=rows, max_vocab=n, k_cap=k, max_history=500)
+        s.set_cluster_rows(0)
+        cd = cands_tensor(rows, k, dev)
+        s.select_rows(lg, params_to_device(p, dev), cd, id_base=base, masks=torch.from_numpy(masks.view(np.int32)).to(dev),
+                      history=torch.from_numpy(h).to(dev), history_len=torch.full((rows,), 500, dtype=torch.int32, device=dev))
+        torch.cuda.synchronize()
+        got = cands_to_numpy(cd)
+        s.close()
+        for r in range(rows):
+            inside = h[r][(h[r] >= base) & (h[r] < base + n)] - base
+            y = oracle.penalize(x[r], inside, None, 1.2, 0.3, 0.2)
+            cv, ci, nk = oracle.topk(y, masks[r], k, base)
+            assert np.array_equal(got["id"][r][:nk], ci[:nk])
+            assert np.array_equal(got["value"][r][:nk].view(np.uint32), (cv[:nk] + np.float32(0.0)).view(np.uint32))
 
 
 def us_per_call(w, dev):
@@ -130,3 +227,22 @@ def test_a_history_that_repeats_itself_costs_little(dev, rows, bf16, masked):
     at = np.minimum((600.0 ** g.random((rows, 2048))).astype(np.int64), 599)
     w.history = np.take_along_axis(ids, at, axis=1)
     assert us_per_call(w, dev) < 1.6 * noise
+
+
+@pytest.mark.parametrize("rows, bf16, masked", [(256, False, True), (1024, True, False)])
+def test_a_history_of_the_best_ids_does_not_cost_a_multiple(dev, rows, bf16, masked):
+    """A row whose best 400 ids are in the history against one whose history is noise.  A bound that could be in the history,
+    lowered step by step and then given up, took 18 and 11.8 times as long; it is 3.2 and 2.4 times."""
+    g, x, w = timed_batch(rows, bf16, masked)
+    noise = us_per_call(w, dev)
+    w.history = hot_history(g, x, w.masks, 2048, 400, 0) if masked else np.tile(hot_history(g, x[:32], None, 2048, 400, 0), (rows // 32, 1))
+    assert us_per_call(w, dev) < 5.0 * noise
+
+
+def test_rows_that_allow_little_do_not_hold_up_a_batch(dev):
+    """k = 128 over rows of which some allow a few hundred to a few thousand ids, too few for a bound from groups of threads:
+    without one for such rows the batch took 184 us, 5 times what it takes when every id is allowed."""
+    _, _, w = timed_batch(128, True, True, k_cap=128)
+    some = us_per_call(w, dev)
+    w.masks = np.full_like(w.masks, 0xFFFFFFFF)
+    assert some < 2.5 * us_per_call(w, dev)

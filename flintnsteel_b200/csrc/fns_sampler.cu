@@ -254,9 +254,13 @@ __device__ int merge_lists(uint64_t * buf, int lists, int len, uint64_t * sel, u
 // serial chains of up to 64 fp64 additions; here every lane holds candidates j = lane and lane + 32 and two warp scans
 // make all running sums together.  A running sum of n <= 64 non-negative terms differs between the two orders by at
 // most 2 n 2^-53 of itself (1.5e-14), a quotient of two of them and one more left-to-right sum by at most 4 n 2^-53
-// (2.9e-14); every comparison is made with kDrawSlack on either side.  That gives the earliest and the latest index at
-// which the left-to-right sums can cut, and from these the earliest and the latest candidate they can pick: if the two
-// are one candidate it is the answer, otherwise (about one draw in 10^11) the caller adds in the reference's order.
+// (2.9e-14).  A caller may have made the weights as exp(d * (1 / T)) where the reference has exp(d / T): two more roundings
+// of an argument of at most 745 in size (past it the weight is 0), so 745 * 2^-52 = 1.7e-13 of the smallest weights.  Every
+// comparison is made with kDrawSlack, several times all of that, on either side.  That gives the earliest and the latest
+// index at which the left-to-right sums can cut, and from these the earliest and the latest candidate they can pick: if the
+// two are one candidate it is the answer, otherwise the caller adds in the reference's order.  How often: a uniform has 24
+// bits, so candidates whose sums lie on its grid (four equal ones: three points of 2^24) or meet top_p exactly ask for it as
+// often as they are hit; sums in general position about once in 10^10 draws.
 // Called by the 32 threads of warp 0.
 constexpr double kDrawSlack = 1e-12;
 __device__ __forceinline__ bool draw_quick(int nk, const double * pj, const double * wj, double u, const fns_b200_params & p, int * pick) {
@@ -1707,12 +1711,12 @@ int fail_cuda(fns_b200_sampler * s, cudaError_t e, const char * where) {
     return FNS_B200_ERR_CUDA;
 }
 
-// Launch geometry.  A block has 512 threads (two fit an SM).  From five rows on a row is one slice: setup, history
-// and draw are paid once per row and there is nothing to merge; this measured faster than any cut at every batch
-// size from 5 to 1024 rows.  Up to four rows are cut into slices of one group per thread (8,192 elements), so that
-// many SMs share the row, and the last block to finish merges the slices' lists.  A slice is a whole number of
-// threads * 16 elements and at most 16 (256 threads) or 32 (512 threads) of them; the slices' lists of one row must
-// fit the merge (kMaxMergeKeys).
+// Launch geometry of k_select.  A block has 512 threads (two fit an SM).  From five rows on a row is one slice: setup,
+// history and draw are paid once per row and there is nothing to merge; for this kernel, whose slices meet in global
+// memory, that measured faster than any cut at every batch size from 5 to 1024 rows.  Up to four rows are cut into slices
+// of one group per thread (8,192 elements), so that many SMs share the row, and the last block to finish merges the
+// slices' lists.  A slice is a whole number of threads * 16 elements and at most 16 (256 threads) or 32 (512 threads) of
+// them; the slices' lists of one row must fit the merge (kMaxMergeKeys).
 bool make_plan_for(const fns_b200_sampler * s, int dtype, int vocab, int rows, int hist_bound, bool aligned, bool whole_rows,
                    Plan & pl) {
     const int k_cap = s->k_cap;
@@ -1751,6 +1755,8 @@ bool make_plan_for(const fns_b200_sampler * s, int dtype, int vocab, int rows, i
     return pl.smem_select <= 200 * 1024;
 }
 
+constexpr size_t kRingTwoPerSm = 115200;  // shared memory of a block of k_ring when two share an SM
+
 // k_ring: one block per row, the row streamed through a ring of shared-memory stages by bulk copies.  Two blocks
 // share an SM when the ring, the bit set and the cell maxima fit twice; a call with no more rows than SMs gives
 // every block an SM of its own and a deeper ring.
@@ -1779,7 +1785,7 @@ bool make_ring_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, 
                         (size_t) kRingThreads * 2 * 8;
     const size_t stage = (size_t) kStageElems * esz;
     // an SM has 228 KB of shared memory and every resident block costs 1 KB on top of what it asks for
-    const size_t two_per_sm = 115200, one_per_sm = 225 * 1024;
+    const size_t two_per_sm = kRingTwoPerSm, one_per_sm = 225 * 1024;
     auto depth_for = [&](size_t budget) -> int {
         if ((size_t) pl.ring_off + tail > budget || (size_t) pl.ring_off + 2 * stage > budget) return 0;
         const size_t d = (budget - pl.ring_off) / stage;
@@ -1818,15 +1824,19 @@ bool make_cluster_plan(const fns_b200_sampler * s, int dtype, int vocab, int his
     return pl.smem_select <= 112 * 1024;  // sixteen of them must be resident together (two fit an SM)
 }
 
-// k_rows: a row cut over `slices` CTAs of one cluster: as many as the chip holds at once (three per SM), while a slice has
-// 32,768 elements or more - below that the two cluster barriers cost what the shorter slices save (64 bf16 rows of V =
-// 151,936: 30 us uncut, 22 in two, 19 in four, 27 in eight; 32 rows of 65,537: 14.8 uncut, 15.6, 17.0, 18.9).
+// k_rows: a row cut over `slices` CTAs of one cluster: as many as the chip holds at once at three per SM, while a slice has
+// 32,768 elements or more (100 fp32 rows of 151,936, every id allowed: 41.9 us uncut, 34.5 in two, 26.8 in four; 32 of 65,537
+// under masks of runs: 16.2 uncut, 15.4 in two, 15.8 in four, where the line was drawn; scattered masks would have it lower:
+// 22.8, 17.3 and 14.8, and 32 rows of 32,000 22.4, 18.9 and 17.4).  In eight only while two such clusters fit every eight SMs: 32 rows of
+// 262,144 take 20.6 us in eight and 26.1 in four, 55 rows 33.6 and 32.0, or under masks of runs 26.5 and 19.3.
 bool make_rows_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, int hist_bound, bool masked, Plan & pl) {
     const int k_cap = s->k_cap;
     const int vec = dtype == FNS_B200_BF16 ? 8 : 4;
     if (k_cap > kRowsMaxK || !s->rows_ok) return false;
     int c = 1;
-    while (2 * c <= kRowsMaxCtas && vocab / (2 * c) >= 32768 && (long long) rows * 2 * c <= 3ll * s->sm_count && kRowsGather / (2 * c) >= k_cap) c *= 2;
+    while (2 * c <= kRowsMaxCtas && vocab / (2 * c) >= 32768 && (long long) rows * 2 * c <= (c < 4 ? 3ll : 2ll) * s->sm_count &&
+           kRowsGather / (2 * c) >= k_cap)
+        c *= 2;
     for (;; c *= 2) {  // (a longer row than one CTA takes is cut further)
         if (c > kRowsMaxCtas || kRowsGather / c < k_cap || (long long) rows * c > 0x7fffffff) return false;
         pl.slices = c;
@@ -1850,12 +1860,15 @@ bool make_rows_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, 
 
 // Batches (from five rows on, what k_cluster does not take) with k_cap up to 128 go to k_rows under a mask, when their rows
 // do not start on 16-byte boundaries, and when there are more of them than six per SM: measured against the kernel that
-// took them before, 256 masked fp32 rows of V = 151,936 take 26.6 us (29.5 in k_select), 64 masked bf16 rows 19.2 us (36),
-// 32 rows of 65,537 side by side 14.8 us (20.4), 1,024 unmasked bf16 rows 99 us (130 in k_ring, whose blocks pay the chain
-// before and after the stream four times).  256 unmasked fp32 rows stay with k_ring: 44 us against 58, the copy engine
-// keeps more bytes under way.  Of the rest, rows without a mask go to k_ring, and any row when k_cap exceeds the 512
-// thread maxima that k_select's bound is made of; k_select has the masked calls with k_cap 129 .. 512, logits read in place
-// from page-locked host memory, forced geometry and the no-allocation entry point.
+// took them before, 256 masked fp32 rows of V = 151,936 take 23.4 us (28.9 in k_select), 64 masked bf16 rows 19.7 us (38),
+// 32 rows of 65,537 side by side 14.2 us (20.8), 1,024 unmasked bf16 rows 99 us (136 in k_ring, whose blocks pay the chain
+// before and after the stream four times).  256 unmasked fp32 rows stay with k_ring: 44 us against 56, the copy engine keeps
+// more bytes under way, and so do more of them while two of its blocks share an SM (1,024 rows of 151,936: 143 us against
+// 154, 896 of them 138 against 137); shorter rows are better off in k_rows (900 rows of 65,536: 75 us against 80, 1,024 rows of
+// 32,000: 58 against 69).
+// Of the rest, rows without a mask go to k_ring, and any row when k_cap exceeds the 512 thread maxima that k_select's bound
+// is made of; k_select has the masked calls with k_cap 129 .. 512, logits read in place from page-locked host memory, forced
+// geometry and the no-allocation entry point.
 bool make_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, int hist_bound, bool aligned, bool masked, Plan & pl) {
     const bool whole_rows = s->force_threads <= 0 && s->force_slices <= 0 && rows > 4;  // (else: sliced rows, if no cluster takes them)
     pl.ring = false;
@@ -1866,7 +1879,12 @@ bool make_plan(const fns_b200_sampler * s, int dtype, int vocab, int rows, int h
         make_cluster_plan(s, dtype, vocab, hist_bound, pl))
         return true;
     pl.cluster = false;
-    if (whole_rows && !s->logits_in_host_memory && (masked || !aligned || rows > 6 * s->sm_count) &&
+    bool many = rows > 6 * s->sm_count;
+    if (many && dtype == FNS_B200_F32 && vocab > 98304) {
+        Plan ring{};
+        many = !make_ring_plan(s, dtype, vocab, rows, hist_bound, ring) || ring.smem_select > kRingTwoPerSm;
+    }
+    if (whole_rows && !s->logits_in_host_memory && (masked || !aligned || many) &&
         make_rows_plan(s, dtype, vocab, rows, hist_bound, masked, pl))
         return true;
     if (whole_rows && aligned && !s->logits_in_host_memory && (!masked || s->k_cap > kRingThreads) &&

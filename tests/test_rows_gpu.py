@@ -246,3 +246,14 @@ def test_rows_that_allow_little_do_not_hold_up_a_batch(dev):
     some = us_per_call(w, dev)
     w.masks = np.full_like(w.masks, 0xFFFFFFFF)
     assert some < 2.5 * us_per_call(w, dev)
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows, slices", [(16, 8), (37, 8), (38, 4), (55, 4)])
+def test_the_longest_rows(dev, oracle, rows, slices, bf16):
+    """V = 262,144 under masks in eight CTAs per row and in four; rows on and off 16-byte boundaries."""
+    g = wl.rng(rows + bf16)
+    for n in (262_144, 262_147):
+        w = batch(g, rows, n, bf16, hist=200, top_hist=True, fractions=(1.0, 0.3, 0.01, 0.003, 0.0005))
+        assert plan_slices(w, 200) == slices
+        check_against_oracle(oracle, w, *run_rows(w, dev, max_history=200, cluster_rows=0))

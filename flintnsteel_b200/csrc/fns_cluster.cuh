@@ -7,11 +7,11 @@
 // maxima pass and the candidate pass both read shared memory, nothing is read twice from global memory, and the
 // history ids' logits are simply looked up in the slice.  The CTAs meet in distributed shared memory, not in global
 // memory:
-//   1. every warp writes the two largest of its threads' maxima into CTA 0 (256 witnesses: distinct elements);
+//   1. every warp writes the two largest of its threads' maxima into every CTA (256 witnesses: distinct elements);
 //      cluster barrier; every CTA finds (nearly) the k-th largest of them by a histogram: a bound that
 //      at least k elements of the row reach
-//   2. every CTA offers the elements of its slice that reach the bound, and its penalised history ids, straight into
-//      CTA 0's candidate buffer (one remote reservation per warp); cluster barrier
+//   2. every CTA gathers the elements of its slice that reach the bound, and its penalised history ids, and stores them into
+//      its own region of CTA 0's candidate buffer (no reservation); cluster barrier
 //   3. CTA 0 ranks the (about k + a few) keys and draws; every CTA has been sent every CTA's number of candidates
 //      together with them, so nobody reads another CTA's memory after the last barrier and none has to wait to leave
 // A mask that leaves too few witnesses for a bound makes every allowed id a candidate: a CTA with more than its region of
@@ -26,7 +26,7 @@ namespace fnsb {
 
 constexpr int kClusterCtas = 16;
 constexpr int kClusterThreads = 256;
-constexpr int kClusterRegion = 128;   // keys a CTA may send to CTA 0 directly; more (from any CTA) means the careful way
+constexpr int kClusterRegion = 128;   // keys a CTA sends to CTA 0; of more it sends its best k
 constexpr int kClusterBuf = kClusterCtas * kClusterRegion;
 constexpr int kClusterLocal = 2048;   // keys of a CTA's own buffer (careful way; in CTA 0 also the regions side by side)
 constexpr int kClusterMaxK = 128;     // 256 witnesses give a bound for k up to this; a region holds k keys

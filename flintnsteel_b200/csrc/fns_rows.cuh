@@ -3,9 +3,10 @@
 //
 // A batch has two bounds: HBM while rows stream, and the chain of dependent steps before and after a row's stream
 // (about 10 us for one block).  So the batch is spread over the whole chip - a row is cut over as many CTAs as fill it,
-// which meet in distributed shared memory - and three CTAs share an SM, whose chains and streams overlap.  The row goes
-// from global memory straight into registers: 128-bit loads, two cells of four vectors in flight per thread, one
-// three-input maximum per two elements, and per cell one 16-bit store that remembers its maximum.
+// which meet in distributed shared memory - and up to three CTAs share an SM, whose chains and streams overlap (registers allow
+// three; an uncut masked fp32 row of 151,936 needs 90 KB of shared memory, of which two fit).  The row goes from global memory
+// straight into registers: 128-bit loads, two cells of four vectors in flight per thread, one three-input maximum per two
+// elements, and per cell one 16-bit store that remembers its maximum.
 //
 //   list     under a mask: the 512-byte segments (what a warp loads with one instruction) that have an allowed id.
 //            Segments that are allowed as a whole are streamed without a look at the bit set; in the others a vector
@@ -14,16 +15,17 @@
 //            (gathering 2,048 logits per row was measured at 13 us of the 62 us that 256 rows took)
 //   bound    256 witnesses per row, each the maximum of one group of lanes.  Without penalties the k-th largest is a
 //            bound: k elements reach it.  With penalties a witness may be a history id, so the bound is a quarter of k
-//            and eight witnesses lower, and it is the count of what was found that proves it
+//            and eight witnesses lower, and it is the count of what was found that proves it.  If it does not, the witnesses
+//            are made again from the cells without a history id (or, where these are few, the bound goes down first)
 //   pass 2   the cells that reach the bound are read again (L2).  What reaches it goes to the CTA's buffer; a history id
 //            among it takes its penalty first, and is dropped if that takes it below the bound.  Penalties that can
 //            raise a value (repetition < 1, negative ones) look at every history id instead
 //   finish   the CTAs send what they have to the row's CTA 0.  k keys or more are proof that the best k are among them:
-//            CTA 0 ranks and draws (rank_draw).  Fewer (many history ids among the best): again with a lower bound
+//            CTA 0 ranks and draws (rank_draw)
 //
 // A row may start on any element: whole vectors start at the first 16-byte boundary, what lies before it (and after the
 // last whole vector) is taken element by element, and the bit sets are read through a funnel shift.
-// Equal values that overflow a list or the buffer send the CTA (alone) through a careful walk with compaction.
+// Equal values, or no bound, may bring more than the buffer holds: the k-th best of a full buffer is then the next bound.
 // No waits but block and hardware cluster barriers.
 #pragma once
 

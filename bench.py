@@ -32,7 +32,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "sampler rows/s (V=151936 fp32, mask+penalties+top-k/p, 256 sessions per GPU)"
 WORKLOAD = "sessions256"
-# dram__bytes_read.sum + dram__bytes_write.sum per k_select launch, from the ncu captures summarised under profiles/
+# dram__bytes_read.sum + dram__bytes_write.sum per k_rows launch (masked) and k_ring launch (dense), from the ncu captures summarised under profiles/
 NCU_TRAFFIC_BYTES = 25.3e6
 NCU_TRAFFIC_BYTES_DENSE = 162.8e6
 
@@ -212,7 +212,7 @@ def run_b200(args):
     sampler.device_status()
 
     # ---- the dominant kernel: its launch duration is the timed region's device time per launch (the region holds
-    # nothing but K back-to-back k_select launches, counted below); event pairs around every single launch, which put
+    # nothing but K back-to-back k_rows launches, counted below); event pairs around every single launch, which put
     # gaps between the launches, are reported beside it
     peak, peak_kind = measured_peaks()
     sel_avg_s = total_ms / max(launches, 1) / 1e3
@@ -325,7 +325,7 @@ def run_b200(args):
                    "parallelism": f"rows{world}"},
         "us_per_row": total_ms * 1e3 / (K * rows),
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "k_select", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "k_ring" if args.no_masks else "k_rows", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": f"of {peak_kind}", "frac_of_8TBps_nominal": achieved / 8000.0,
                      "bytes_per_launch": rows * row_bytes, "avg_launch_us": sel_avg_s * 1e6,
                      "isolated_launch_us": isolated_us,
